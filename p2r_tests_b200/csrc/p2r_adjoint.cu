@@ -467,7 +467,7 @@ __device__ __forceinline__ void rev_track_ck1(const AdjParams& p, const TrackCtx
       for (int i = 0; i < 21; ++i) cb[i] = cin[i];
       drb = rbar;
       if (rh > T(0)) {
-        const T irh = T(1) / rh;
+        const T irh = adj::rcp_(rh);
         hpb[0] += rbar * hp[0] * irh;
         hpb[1] += rbar * hp[1] * irh;
       }
