@@ -19,6 +19,9 @@ from ._lib import P2RError, check, lib
 from .api import Config, HIT_WORDS, TRK_WORDS, _arg, _check_shapes, _ptr, _stream
 
 
+_SMALL_WORKSPACE = 256 << 20  # 0.15 % of the device memory; about 60000 tracks x 20 layers
+
+
 def workspace_size(cfg: Config, ckpt_stride: int | None = None) -> int:
     """Workspace bytes of p2r_forward_backward: the minimum (checkpoints in thread-local
     memory) when ckpt_stride is None, else the size that also holds the checkpoint tape."""
@@ -35,11 +38,16 @@ def workspace_size(cfg: Config, ckpt_stride: int | None = None) -> int:
 def auto_ckpt_stride(cfg: Config, device, tape: bool = True) -> int:
     """The checkpoint stride used when the caller names none: 1 (the whole state tape, the
     fastest reverse) when its workspace fits in half the free device memory, else 5; 5 for
-    thread-local checkpoints."""
+    thread-local checkpoints. A workspace of at most _SMALL_WORKSPACE is taken to fit: asking the
+    driver for the free memory takes 70 us, and 255 us while kernels run, as long as the whole
+    forward + adjoint of 9600 tracks."""
     if not tape:
         return 5
+    need = workspace_size(cfg, 1)
+    if need <= _SMALL_WORKSPACE:
+        return 1
     free, _ = torch.cuda.mem_get_info(device)
-    return 1 if workspace_size(cfg, 1) <= free // 2 else 5
+    return 1 if need <= free // 2 else 5
 
 
 def forward_backward(cfg: Config, trk_in, hits, dr=None, nlay_lane=None, grad_trk_out=None, grad_chi2=None,
@@ -54,25 +62,32 @@ def forward_backward(cfg: Config, trk_in, hits, dr=None, nlay_lane=None, grad_tr
     _check_shapes(cfg, trk_in, hits)
     dev = trk_in.device
     o = out if out is not None else {}
-    if ckpt_stride is None:
+    chosen = ckpt_stride is None
+    if chosen:
         if o.get("ckpt_stride") is None:
             o["ckpt_stride"] = auto_ckpt_stride(cfg, dev, tape)
         ckpt_stride = o["ckpt_stride"]
-    f32 = dict(dtype=torch.float32, device=dev)
-    f64 = dict(dtype=torch.float64, device=dev)
-    o.setdefault("trk_out", torch.empty_like(trk_in))
-    o.setdefault("chi2", torch.empty(cfg.ntracks, **f32))
-    o.setdefault("grad_trk_in", torch.empty_like(trk_in))
-    o.setdefault("grad_hits", torch.empty_like(hits))
-    o.setdefault("grad_dr", torch.empty(cfg.nlayer, **f64))
-    o.setdefault("grad_bz", torch.empty(1, **f64))
+    f32, f64 = torch.float32, torch.float64
+    for name, like in (("trk_out", trk_in), ("grad_trk_in", trk_in), ("grad_hits", hits)):
+        if name not in o:
+            o[name] = torch.empty_like(like)
+    sizes = [("chi2", (cfg.ntracks,), f32), ("grad_dr", (cfg.nlayer,), f64), ("grad_bz", (1,), f64)]
     if per_event:
-        o.setdefault("grad_dr_event", torch.empty(cfg.nevts, cfg.nlayer, **f64))
-        o.setdefault("grad_bz_event", torch.empty(cfg.nevts, **f64))
+        sizes += [("grad_dr_event", (cfg.nevts, cfg.nlayer), f64), ("grad_bz_event", (cfg.nevts,), f64)]
+    for name, shape, dtype in sizes:
+        if name not in o:
+            o[name] = torch.empty(shape, dtype=dtype, device=dev)
     ws = o.get("workspace")
     need = workspace_size(cfg, ckpt_stride if tape else None)
     if ws is None or ws.numel() < need:
-        ws = torch.empty(need, dtype=torch.uint8, device=dev)
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=dev)
+        except torch.cuda.OutOfMemoryError:
+            if not chosen or not tape or ckpt_stride != 1:
+                raise
+            ckpt_stride = o["ckpt_stride"] = 5  # a fifth of the tape
+            need = workspace_size(cfg, ckpt_stride)
+            ws = torch.empty(need, dtype=torch.uint8, device=dev)
         o["workspace"] = ws
     c = cfg.c()
     ntrk, nt, nh, nl = cfg.ntracks, trk_in.numel(), hits.numel(), cfg.nlayer
@@ -112,7 +127,8 @@ class P2RChain(torch.autograd.Function):
         trk, hits, dr = ctx.saved_tensors
         g_trk_out = None if g_trk_out is None else g_trk_out.contiguous()
         g_chi2 = None if g_chi2 is None else g_chi2.contiguous()
+        # trk_out and chi2 are the forward's already
         o = forward_backward(ctx.cfg, trk, hits, dr=dr, grad_trk_out=g_trk_out, grad_chi2=g_chi2,
-                             ckpt_stride=ctx.ckpt)
+                             ckpt_stride=ctx.ckpt, out={"trk_out": None, "chi2": None})
         return (o["grad_trk_in"], o["grad_hits"], o["grad_dr"].to(dr.dtype),
                 o["grad_bz"][0].to(dtype=ctx.bz_dtype, device=ctx.bz_device), None, None)
