@@ -28,6 +28,7 @@
 
 #include "p2r_adjoint.cuh"
 #include "p2r_internal.h"
+#include "p2r_launch.cuh"
 #include "p2r_queue_check.cuh"
 
 namespace p2r {
@@ -73,6 +74,7 @@ __device__ __forceinline__ void load_hit_t(const float* h, int bs, int it, T (&h
 // T: arithmetic type of the whole kernel (float or double). CK: checkpoint stride.
 template <class T, int CK>
 __global__ void __launch_bounds__(kAdjThreads) fwdbwd_kernel(AdjParams p) {
+  pdl_wait();
   constexpr int NCK = (kMaxAdjLayers + CK - 1) / CK;
   const int bs = p.bsize;
   const int lane = threadIdx.x & 31;
@@ -483,6 +485,7 @@ __device__ __forceinline__ void rev_track_ck1(const AdjParams& p, const TrackCtx
 
 template <class T, int CK>
 __global__ void __launch_bounds__(kAdjThreads) fwd_tape_kernel(AdjParams p, TapeParams tp) {
+  pdl_wait();
   T par[6], cov[21];
   long long g;
   const TrackCtx<T> c = grid_track(p, par, cov, g);
@@ -504,6 +507,7 @@ __global__ void __launch_bounds__(kAdjThreads) fwd_tape_kernel(AdjParams p, Tape
 
 template <class T, int CK>
 __global__ void __launch_bounds__(kAdjThreads) rev_tape_kernel(AdjParams p, TapeParams tp) {
+  pdl_wait();
   T par[6], cov[21];
   long long g;
   const TrackCtx<T> c = grid_track(p, par, cov, g);
@@ -581,6 +585,7 @@ struct QAdjParams {
 
 __global__ void __launch_bounds__(kAdjThreads) queue_adj_kernel(AdjParams p, QAdjParams q) {
   __shared__ long long s_item;
+  pdl_wait();
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int spb = p.bsize / 32;
@@ -641,6 +646,7 @@ __global__ void __launch_bounds__(kOrderThreads) order_by_layers_kernel(const in
   constexpr int kW = kOrderThreads / 32;
   __shared__ int base[kMaxAdjLayers + 1];
   __shared__ int wcount[kW][kMaxAdjLayers + 1];
+  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nkeys = nlayer + 1;
   const long long e = blockIdx.x;
@@ -714,6 +720,7 @@ inline dim3 order_grid(long long nevts) {
 __global__ void __launch_bounds__(256) sum_partials_kernel(const double* partials, long long nwarps, int nout,
                                                            long long wpe, double* out) {
   __shared__ double red[256];
+  pdl_wait();
   const long long e = blockIdx.x;
   const int j = blockIdx.y;
   const long long w0 = e * wpe, w1 = min(w0 + wpe, nwarps);
@@ -728,24 +735,43 @@ __global__ void __launch_bounds__(256) sum_partials_kernel(const double* partial
   if (threadIdx.x == 0) out[e * nout + j] = red[0];
 }
 
-// out[j] = sum over rows of in[rows][nout], fixed order.
-__global__ void sum_rows_kernel(const double* in, long long rows, int nout, double* out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nout) return;
+// Outputs of the shared gradients from the per-event sums ev[rows][nlayer + 1]: block j writes column j
+// to the event outputs and its sum over the rows, added in their order, to the totals (one launch for
+// what took three, 22 us of them at 100 events: the rows are loaded together and only the additions
+// are serial).
+__global__ void __launch_bounds__(256) finish_kernel(const double* ev, long long rows, int nlayer, double* tot,
+                                                     double* g_dr, double* g_bz, double* g_dr_event,
+                                                     double* g_bz_event) {
+  __shared__ double col[256];
+  pdl_wait();
+  const int j = blockIdx.x, nout = nlayer + 1;
   double s = 0.0;
-  for (long long r = 0; r < rows; ++r) s += in[r * nout + j];
-  out[j] = s;
-}
-
-__global__ void split_kernel(const double* src, long long rows, int nlayer, double* g_dr, double* g_bz) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * (nlayer + 1)) return;
-  const long long r = i / (nlayer + 1);
-  const int j = (int)(i - r * (nlayer + 1));
-  if (j < nlayer) {
-    if (g_dr) g_dr[r * nlayer + j] = src[i];
-  } else if (g_bz) {
-    g_bz[r] = src[i];
+  for (long long r0 = 0; r0 < rows; r0 += 256) {
+    const long long r = r0 + threadIdx.x;
+    if (r < rows) {
+      const double v = ev[r * nout + j];
+      col[threadIdx.x] = v;
+      if (j < nlayer) {
+        if (g_dr_event) g_dr_event[r * nlayer + j] = v;
+      } else if (g_bz_event) {
+        g_bz_event[r] = v;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int n = (int)(rows - r0 < 256 ? rows - r0 : 256);
+#pragma unroll 8
+      for (int k = 0; k < n; ++k) s += col[k];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    tot[j] = s;
+    if (j < nlayer) {
+      if (g_dr) g_dr[j] = s;
+    } else if (g_bz) {
+      *g_bz = s;
+    }
   }
 }
 
@@ -800,10 +826,9 @@ int normal_ckpt(int ckpt_stride) { return ckpt_stride == 0 ? 5 : ckpt_stride; }
 
 template <class T, int CK>
 cudaError_t launch_tape(const AdjParams& p, const TapeParams& tp, cudaStream_t st) {
-  const unsigned grid = (unsigned)(tp.nthreads / kAdjThreads);
-  fwd_tape_kernel<T, CK><<<grid, kAdjThreads, 0, st>>>(p, tp);
-  rev_tape_kernel<T, CK><<<grid, kAdjThreads, 0, st>>>(p, tp);
-  return cudaGetLastError();
+  const dim3 grid((unsigned)(tp.nthreads / kAdjThreads));
+  const cudaError_t e = launch_pdl(fwd_tape_kernel<T, CK>, grid, kAdjThreads, 0, st, p, tp);
+  return e != cudaSuccess ? e : launch_pdl(rev_tape_kernel<T, CK>, grid, kAdjThreads, 0, st, p, tp);
 }
 
 template <class T>
@@ -820,8 +845,7 @@ cudaError_t launch_tape_ck(const AdjParams& p, const TapeParams& tp, int ck, cud
 template <class T, int CK>
 cudaError_t launch_fwdbwd(const AdjParams& p, long long ntr, cudaStream_t st) {
   const long long grid = (ntr + kAdjThreads - 1) / kAdjThreads;
-  fwdbwd_kernel<T, CK><<<(unsigned)grid, kAdjThreads, 0, st>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(fwdbwd_kernel<T, CK>, dim3((unsigned)grid), kAdjThreads, 0, st, p);
 }
 
 template <class T>
@@ -933,10 +957,8 @@ int p2r_forward_backward(const p2r_config* cfg, const void* trk_in, const void* 
     return p2r_set_errorf(P2R_ERR_UNSUPPORTED, "%s: checkpoint stride %d (use 1, 2, 4, 5 or 10)", who, ckpt_stride);
   if (ordered) {
     const long long win = kOrderWindow / cfg->bsize > 0 ? kOrderWindow / cfg->bsize : 1;
-    order_by_layers_kernel<<<order_grid(cfg->nevts), kOrderThreads, 0, st>>>(nlay_lane, nullptr, cfg->nb, nblocks,
-                                                                           cfg->bsize, cfg->nlayer, win,
-                                                                           (uint32_t*)p.order);
-    e = cudaGetLastError();
+    e = launch_pdl(order_by_layers_kernel, order_grid(cfg->nevts), kOrderThreads, 0, st, nlay_lane,
+                   (const int64_t*)nullptr, cfg->nb, nblocks, cfg->bsize, cfg->nlayer, win, (uint32_t*)p.order);
     if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
   }
   const bool fp32 = (cfg->flags & P2R_FLAG_ADJ_FP32) != 0;
@@ -957,18 +979,14 @@ int p2r_forward_backward(const p2r_config* cfg, const void* trk_in, const void* 
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
   const int nout = cfg->nlayer + 1;
   double* ev = (double*)((char*)workspace + w.event_off);
-  double* tot = (double*)((char*)workspace + w.total_off);
-  // per-event sums (warps of an event are contiguous when bsize % 32 == 0), then totals
+  // per-event sums (warps of an event are contiguous when bsize % 32 == 0), then totals and outputs
   const bool per_event = cfg->bsize % 32 == 0;
   const long long wpe = per_event ? cfg->nb * cfg->bsize / 32 : w.nwarps;
   const long long rows = per_event ? cfg->nevts : 1;
-  sum_partials_kernel<<<dim3((unsigned)rows, (unsigned)nout), 256, 0, st>>>(p.partials, w.nwarps, nout, wpe, ev);
-  sum_rows_kernel<<<(nout + 63) / 64, 64, 0, st>>>(ev, rows, nout, tot);
-  if (grad_dr || grad_bz) split_kernel<<<(nout + 63) / 64, 64, 0, st>>>(tot, 1, cfg->nlayer, grad_dr, grad_bz);
-  if (grad_dr_event || grad_bz_event)
-    split_kernel<<<(unsigned)((rows * nout + 255) / 256), 256, 0, st>>>(ev, rows, cfg->nlayer, grad_dr_event,
-                                                                        grad_bz_event);
-  e = cudaGetLastError();
+  e = launch_pdl(sum_partials_kernel, dim3((unsigned)rows, (unsigned)nout), 256, 0, st, p.partials, w.nwarps, nout, wpe, ev);
+  if (e == cudaSuccess)
+    e = launch_pdl(finish_kernel, dim3((unsigned)nout), 256, 0, st, ev, rows, cfg->nlayer,
+                   (double*)((char*)workspace + w.total_off), grad_dr, grad_bz, grad_dr_event, grad_bz_event);
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "%s: reduction launch failed: %s", who, cudaGetErrorString(e));
   return p2r_clear_error();
 }
@@ -1102,6 +1120,7 @@ namespace p2r {
 __global__ void __launch_bounds__(256) sum_slices_kernel(const double* partials, const int64_t* ev_off,
                                                          long long nblocks, int spb, int nout, double* out) {
   __shared__ double red[256];
+  pdl_wait();
   const long long e = blockIdx.x;
   const int j = blockIdx.y;
   long long b0 = ev_off[e], b1 = ev_off[e + 1];
@@ -1261,26 +1280,20 @@ int enqueue_queue_adjoint(const p2r_queue* q, const void* trk_in, const void* hi
   if (e == cudaSuccess && w.nslices > 0)
     e = cudaMemsetAsync(qp.slice_partials, 0, (size_t)w.nslices * (q->nlayer + 1) * sizeof(double), st);
   if (e == cudaSuccess && qp.order && q->nblocks > 0) {
-    order_by_layers_kernel<<<order_grid(q->nevts), kOrderThreads, 0, st>>>(
-        q->nlay_lane, q->event_block_offset, 0, q->nblocks, q->bsize, q->nlayer, 0, (uint32_t*)qp.order);
-    e = cudaGetLastError();
+    e = launch_pdl(order_by_layers_kernel, order_grid(q->nevts), kOrderThreads, 0, st, q->nlay_lane,
+                   q->event_block_offset, 0LL, q->nblocks, q->bsize, q->nlayer, 0LL, (uint32_t*)qp.order);
   }
   if (e == cudaSuccess && q->n_items > 0) {
-    queue_adj_kernel<<<(unsigned)grid, threads, 0, st>>>(p, qp);
-    e = cudaGetLastError();
+    e = launch_pdl(queue_adj_kernel, dim3((unsigned)grid), threads, 0, st, p, qp);
   }
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
   const int nout = q->nlayer + 1;
   double* ev = (double*)((char*)workspace + w.event_off);
-  double* tot = (double*)((char*)workspace + w.total_off);
-  sum_slices_kernel<<<dim3((unsigned)q->nevts, (unsigned)nout), 256, 0, st>>>(
-      qp.slice_partials, q->event_block_offset, q->nblocks, q->bsize / 32, nout, ev);
-  sum_rows_kernel<<<(nout + 63) / 64, 64, 0, st>>>(ev, q->nevts, nout, tot);
-  if (grad_dr || grad_bz) split_kernel<<<(nout + 63) / 64, 64, 0, st>>>(tot, 1, q->nlayer, grad_dr, grad_bz);
-  if (grad_dr_event || grad_bz_event)
-    split_kernel<<<(unsigned)((q->nevts * nout + 255) / 256), 256, 0, st>>>(ev, q->nevts, q->nlayer, grad_dr_event,
-                                                                            grad_bz_event);
-  e = cudaGetLastError();
+  e = launch_pdl(sum_slices_kernel, dim3((unsigned)q->nevts, (unsigned)nout), 256, 0, st, qp.slice_partials,
+                 q->event_block_offset, q->nblocks, q->bsize / 32, nout, ev);
+  if (e == cudaSuccess)
+    e = launch_pdl(finish_kernel, dim3((unsigned)nout), 256, 0, st, ev, q->nevts, q->nlayer,
+                   (double*)((char*)workspace + w.total_off), grad_dr, grad_bz, grad_dr_event, grad_bz_event);
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "%s: reduction launch failed: %s", who, cudaGetErrorString(e));
   return p2r_clear_error();
 }

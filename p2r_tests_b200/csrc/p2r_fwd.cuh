@@ -16,6 +16,7 @@
 #include <stdint.h>
 
 #include "p2r_internal.h"
+#include "p2r_launch.cuh"
 #include "p2r_math.cuh"
 
 namespace p2r {
@@ -131,6 +132,7 @@ __device__ __forceinline__ void chained_slice_staged(const FwdParams& p, long lo
 template <int BS, int STAGES, bool STAGED, bool RESTART, bool CHI2, bool DR, bool MASK, bool FP64DET, bool SQUASH>
 __global__ void __launch_bounds__(128) fwd_kernel(FwdParams p) {
   extern __shared__ __align__(16) float smem[];
+  pdl_wait();
   const int bs = BS > 0 ? BS : p.bsize;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long b = g / bs;
@@ -233,8 +235,7 @@ inline cudaError_t launch_fwd(const FwdParams& p, int threads, cudaStream_t st) 
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<(unsigned)grid, threads, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)grid), threads, smem, st, p);
 }
 
 // compile-time bsize dispatch

@@ -8,6 +8,7 @@ namespace p2r {
 template <int BS, int NW, bool CHI2, bool DR, bool SQUASH>
 __global__ void __launch_bounds__(NW * 32, kOrdWarpsPerSm / NW) fwd_ordered_kernel(FwdParams p) {
   __shared__ OrdSmem<NW> sm;
+  pdl_wait();
   const int bs = BS > 0 ? BS : p.bsize;
   const int cb = ordered_chunk_blocks<NW>(bs);
   const long long b0 = (long long)blockIdx.x * cb;
@@ -19,8 +20,7 @@ template <int BS, int NW, bool CHI2, bool DR, bool SQUASH>
 cudaError_t launch_ordered_t(const FwdParams& p, cudaStream_t st) {
   const int cb = ordered_chunk_blocks<NW>(p.bsize);
   const long long grid = (p.nblocks + cb - 1) / cb;
-  fwd_ordered_kernel<BS, NW, CHI2, DR, SQUASH><<<(unsigned)grid, NW * 32, 0, st>>>(p);
-  return cudaGetLastError();
+  return launch_pdl(fwd_ordered_kernel<BS, NW, CHI2, DR, SQUASH>, dim3((unsigned)grid), NW * 32, 0, st, p);
 }
 
 template <int NW, bool CHI2, bool DR, bool SQUASH>

@@ -45,6 +45,7 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 
 __global__ void queue_init_kernel(const int64_t* ev_off, long long nevts, long long nblocks, int slices_per_block,
                                   int* counter, int* ev_remaining, unsigned* error, unsigned long long* t_start) {
+  pdl_wait();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e == 0) {
     *counter = 0;
@@ -66,6 +67,7 @@ template <int BS, int STAGES, bool CHI2, bool FP64DET, bool SQUASH>
 __global__ void __launch_bounds__(128) queue_kernel(QueueParams q) {
   extern __shared__ __align__(16) float smem[];
   __shared__ int s_item;
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int bs = BS > 0 ? BS : q.f.bsize;
   const int spb = bs / 32;  // 32-lane slices per block
@@ -105,6 +107,7 @@ template <int BS, int NW, bool CHI2, bool FP64DET, bool SQUASH>
 __global__ void __launch_bounds__(NW * 32, kOrdWarpsPerSm / NW) queue_ordered_kernel(QueueParams q) {
   __shared__ OrdSmem<NW> sm;
   __shared__ long long s_item;
+  pdl_wait();
   const FwdParams& p = q.f;
   const int bs = BS > 0 ? BS : p.bsize;
   const int spb = bs / 32;
@@ -147,8 +150,7 @@ cudaError_t launch_queue_ordered_t(const QueueParams& q, int ctas_per_sm, cudaSt
   const int per_sm = ctas_per_sm > 0 ? (ctas_per_sm < occ ? ctas_per_sm : occ) : occ;
   const long long want = (long long)sms * (per_sm > 0 ? per_sm : 1);
   const long long grid = want < q.n_items ? want : (q.n_items > 0 ? q.n_items : 1);
-  kern<<<(unsigned)grid, kOrdThreads, 0, st>>>(q);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)grid), kOrdThreads, 0, st, q);
 }
 
 template <int NW, bool CHI2, bool FP64DET, bool SQUASH>
@@ -173,8 +175,7 @@ cudaError_t launch_queue_t(const QueueParams& q, int threads, int ctas_per_sm, c
   const int per_sm = ctas_per_sm > 0 ? (ctas_per_sm < occ ? ctas_per_sm : occ) : occ;
   const long long want = (long long)sms * (per_sm > 0 ? per_sm : 1);
   const long long grid = want < q.n_items ? want : (q.n_items > 0 ? q.n_items : 1);
-  kern<<<(unsigned)grid, threads, smem, st>>>(q);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)grid), threads, smem, st, q);
 }
 
 template <int STAGES, bool CHI2, bool FP64DET, bool SQUASH>
@@ -298,9 +299,8 @@ int enqueue_queue(const p2r_queue* q, const void* trk_in, const void* hits, void
   // the error word is cleared before any kernel of this launch can set a bit
   cudaError_t e = cudaMemsetAsync(qp.error, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
-  queue_init_kernel<<<(unsigned)((q->nevts + 255) / 256), 256, 0, st>>>(
-      q->event_block_offset, q->nevts, q->nblocks, q->bsize / 32, qp.counter, qp.ev_remaining, qp.error, start_ns);
-  e = cudaGetLastError();
+  e = launch_pdl(queue_init_kernel, dim3((unsigned)((q->nevts + 255) / 256)), 256, 0, st, q->event_block_offset, q->nevts,
+                 q->nblocks, q->bsize / 32, qp.counter, qp.ev_remaining, qp.error, start_ns);
   if (e == cudaSuccess) {
     const int threads = q->block_threads > 0 ? q->block_threads : 128;
     const int stages = q->stages > 0 ? q->stages : 4;
