@@ -206,13 +206,26 @@ __global__ void __launch_bounds__(128) fwd_kernel(FwdParams p) {
     }
     cp_async_wait<0>();
   } else {
+    // Any bsize and alignment: a lane reads its own track's hits, the next layer's in flight while the
+    // current one computes (loaded at the top of each layer instead, 400000 tracks x 20 layers at bsize
+    // 20 take 198 us, so 195; 160 tracks 20.6 -> 18.5 us: B200).
+    const float* h = hblk + it;
+    float hn[9];
+    if (nl > 0) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) hn[i] = __ldcs(h + i * bs);
+    }
     for (int l = 0; l < nl; ++l) {
-      const float* h = hblk + (long long)l * (kHitWords * bs);
       float hp[3], hc[6];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) hp[i] = __ldcs(h + i * bs + it);
+      for (int i = 0; i < 3; ++i) hp[i] = hn[i];
 #pragma unroll
-      for (int i = 0; i < 6; ++i) hc[i] = __ldcs(h + (3 + i) * bs + it);
+      for (int i = 0; i < 6; ++i) hc[i] = hn[3 + i];
+      if (l + 1 < nl) {  // the next layer's hit, in flight while this layer computes
+        h += kHitWords * bs;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) hn[i] = __ldcs(h + i * bs);
+      }
       const float rh = hipo(hp[0], hp[1]);
       const float rt = DR ? rh + __ldg(p.dr + l) : rh;
       propagate_to_r(par, cov, k, kinv, rt, par, cov);
