@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(128) fwd_kernel(FwdParams p) {
       if (!MASK || l < nl) {
         const float rh = hipo(hp[0], hp[1]);
         const float rt = DR ? rh + __ldg(p.dr + l) : rh;
-        propagate_to_r(par, cov, k, kinv, rt, par, cov);
+        propagate_to_r<!MASK>(par, cov, k, kinv, rt, par, cov);
         chi2 += kalman_update<FP64DET, CHI2>(par, cov, hp, hc, rh);
         if (SQUASH) par[4] = squash_phi(par[4]);
       }
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(128) fwd_kernel(FwdParams p) {
       }
       const float rh = hipo(hp[0], hp[1]);
       const float rt = DR ? rh + __ldg(p.dr + l) : rh;
-      propagate_to_r(par, cov, k, kinv, rt, par, cov);
+      propagate_to_r<!MASK>(par, cov, k, kinv, rt, par, cov);
       chi2 += kalman_update<FP64DET, CHI2>(par, cov, hp, hc, rh);
       if (SQUASH) par[4] = squash_phi(par[4]);
     }
