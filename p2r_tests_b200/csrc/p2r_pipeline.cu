@@ -1,12 +1,22 @@
-// Host-buffer driver: events split into chunks whose host->device copy, fused forward and
+// Host-buffer driver: the track blocks split into chunks whose host->device copy, fused forward and
 // device->host copy run on a small pool of streams, so the copies of one chunk overlap the
 // kernel of another. This is the transfer pipeline of the reference's multi-stream CUDA
 // driver (cuda_v4.cu:912-1010: per-stream cudaMemcpyAsync H2D, kernel, D2H), over the same
-// Matriplex arrays. Events are contiguous in both arrays (track block ib + nb*ev, hit block
-// lay + nlayer*(ib + nb*ev)), so a chunk of events is one contiguous byte range of each.
+// Matriplex arrays. Track blocks and their hit blocks are contiguous in both arrays (track block
+// ib + nb*ev, hit block lay + nlayer*(ib + nb*ev)) and independent, so any range of blocks is one
+// contiguous byte range of each.
 // In restart mode only the last layer reaches the output (the reference's restart loop
 // rewrites it at every layer from the same input track), so only that layer's hit block of
 // each track block is copied: one strided 2-D copy per chunk, a 1/nlayer share of the hits.
+//
+// The host link bounds the call (55.5 GB/s host->device); every gap between two copies and the last
+// chunk's kernel and copy back come on top. So chunks are equal numbers of blocks, but the last is a
+// quarter of the others; none is below 4 MiB, where a copy costs more than it hides; and in chained
+// mode the tracks (one byte in seven at 20 layers) go over in one copy before the hits.
+// Measured on one B200, pinned buffers, 8 chunks asked for, chunks of whole events before -> this:
+// 9600 x 10 x 20 1617 -> 1541 us (80 MB in, 1440 us at the link's rate), 9600 x 60 x 20 9.34 -> 8.83 ms,
+// 5000 x 7 x 12 470 -> 428 us, 9600 x 1 x 20 203 -> 201 us; restart 9600 x 10 505 -> 440 us. Tracks in
+// one copy in restart mode too, where they are most of the bytes: 9600 x 60 2.1 -> 2.5 ms.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -17,6 +27,8 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 constexpr int kPoolStreams = 3;
+constexpr size_t kMinChunkBytes = size_t(4) << 20;  // host->device bytes of a chunk
+constexpr int kLastShare = 4;                       // the last chunk is 1 / kLastShare of another
 
 struct StreamPool {
   std::mutex mu;  // one call at a time enqueues on the pool (the fork / join events are shared)
@@ -82,12 +94,16 @@ extern "C" int p2r_forward_host(const p2r_config* cfg, const void* host_trk_in, 
   StreamPool* pool = nullptr;
   if ((rc = get_pool(&pool))) return rc;
   std::lock_guard<std::mutex> lk(pool->mu);
-  const int64_t chunks = nchunks > cfg->nevts ? cfg->nevts : nchunks;
-  const size_t trk_ev = (size_t)cfg->nb * 28 * cfg->bsize * sizeof(float);
-  const size_t hit_ev = (size_t)cfg->nb * cfg->nlayer * 9 * cfg->bsize * sizeof(float);
+  const int64_t nblocks = (int64_t)cfg->nevts * cfg->nb;
+  const size_t trk_blk = (size_t)28 * cfg->bsize * sizeof(float);
   const size_t hit_blk = (size_t)9 * cfg->bsize * sizeof(float);  // one layer of one track block
+  const size_t hit_trk = (size_t)cfg->nlayer * hit_blk;                // all layers of one track block
   const size_t last = (size_t)(cfg->nlayer - 1) * hit_blk;          // offset of the last layer's block
   const bool restart = cfg->mode == P2R_MODE_RESTART;
+  const size_t total = (size_t)nblocks * (trk_blk + (restart ? hit_blk : hit_trk));
+  int64_t chunks = (int64_t)(total / kMinChunkBytes);
+  chunks = chunks < 1 ? 1 : (chunks > nchunks ? nchunks : chunks);
+  if (chunks > nblocks) chunks = nblocks;
   cudaStream_t caller = (cudaStream_t)stream;
   cudaError_t e = cudaEventRecord(pool->fork, caller);
   for (int i = 0; i < kPoolStreams && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(pool->s[i], pool->fork, 0);
@@ -101,31 +117,43 @@ extern "C" int p2r_forward_host(const p2r_config* cfg, const void* host_trk_in, 
     }
     return je;
   };
+  const bool tracks_first = !restart && chunks > 1;
+  if (tracks_first) {
+    if ((e = cudaMemcpyAsync(dev_trk_in, host_trk_in, nblocks * trk_blk, cudaMemcpyHostToDevice, pool->s[0])) == cudaSuccess &&
+        (e = cudaEventRecord(pool->join[0], pool->s[0])) == cudaSuccess)
+      for (int i = 1; i < kPoolStreams && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(pool->s[i], pool->join[0], 0);
+    if (e != cudaSuccess) {
+      join();
+      return p2r_set_errorf(P2R_ERR_CUDA, "p2r_forward_host: H2D: %s", cudaGetErrorString(e));
+    }
+  }
+  const int64_t step = chunks > 2 ? kLastShare : 1;
+  const int64_t parts = step * (chunks - 1) + 1;
   for (int64_t c = 0; c < chunks; ++c) {
-    const int64_t ev0 = cfg->nevts * c / chunks, ev1 = cfg->nevts * (c + 1) / chunks;
-    if (ev1 == ev0) continue;
+    const int64_t b0 = nblocks * (step * c) / parts, b1 = c + 1 == chunks ? nblocks : nblocks * (step * (c + 1)) / parts;
+    if (b1 == b0) continue;
+    const int64_t nb = b1 - b0;
     cudaStream_t s = pool->s[c % kPoolStreams];
-    char* dti = (char*)dev_trk_in + ev0 * trk_ev;
-    char* dh = (char*)dev_hits + ev0 * hit_ev;
-    char* dto = (char*)dev_trk_out + ev0 * trk_ev;
-    if ((e = cudaMemcpyAsync(dti, (const char*)host_trk_in + ev0 * trk_ev, (ev1 - ev0) * trk_ev,
-                             cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = restart ? cudaMemcpy2DAsync(dh + last, (size_t)cfg->nlayer * hit_blk,
-                                         (const char*)host_hits + ev0 * hit_ev + last, (size_t)cfg->nlayer * hit_blk,
-                                         hit_blk, (size_t)(ev1 - ev0) * cfg->nb, cudaMemcpyHostToDevice, s)
-                     : cudaMemcpyAsync(dh, (const char*)host_hits + ev0 * hit_ev, (ev1 - ev0) * hit_ev,
-                                       cudaMemcpyHostToDevice, s)) != cudaSuccess)
-    {
+    char* dti = (char*)dev_trk_in + b0 * trk_blk;
+    char* dh = (char*)dev_hits + b0 * hit_trk;
+    char* dto = (char*)dev_trk_out + b0 * trk_blk;
+    if ((!tracks_first && (e = cudaMemcpyAsync(dti, (const char*)host_trk_in + b0 * trk_blk, nb * trk_blk,
+                                               cudaMemcpyHostToDevice, s)) != cudaSuccess) ||
+        (e = restart ? cudaMemcpy2DAsync(dh + last, hit_trk, (const char*)host_hits + b0 * hit_trk + last, hit_trk, hit_blk,
+                                         (size_t)nb, cudaMemcpyHostToDevice, s)
+                     : cudaMemcpyAsync(dh, (const char*)host_hits + b0 * hit_trk, nb * hit_trk, cudaMemcpyHostToDevice,
+                                       s)) != cudaSuccess) {
       join();
       return p2r_set_errorf(P2R_ERR_CUDA, "p2r_forward_host: H2D: %s", cudaGetErrorString(e));
     }
     p2r_config sub = *cfg;
-    sub.nevts = ev1 - ev0;
+    sub.nevts = 1;
+    sub.nb = nb;
     if ((rc = p2r_forward(&sub, dti, dh, dto, nullptr, nullptr, s))) {
       join();
       return rc;
     }
-    if ((e = cudaMemcpyAsync((char*)host_trk_out + ev0 * trk_ev, dto, (ev1 - ev0) * trk_ev, cudaMemcpyDeviceToHost,
+    if ((e = cudaMemcpyAsync((char*)host_trk_out + b0 * trk_blk, dto, nb * trk_blk, cudaMemcpyDeviceToHost,
                              s)) != cudaSuccess) {
       join();
       return p2r_set_errorf(P2R_ERR_CUDA, "p2r_forward_host: D2H: %s", cudaGetErrorString(e));
