@@ -68,7 +68,9 @@ typedef enum p2r_mode { P2R_MODE_RESTART = 0, P2R_MODE_CHAINED = 1 } p2r_mode;
                                     track's own position and every track's result is the same
                                     arithmetic (shared gradient sums are added in the new grouping).
                                     p2r_forward_masked (cfg.flags): within each CTA's chunk of 256 or
-                                    512 tracks (FP64 determinant, nlayer <= 64, bsize <= 512); the
+                                    512 tracks (FP64 determinant, nlayer <= 64, bsize <= 512), in batches
+                                    that fill the GPU (smaller ones are not ordered: same results,
+                                    sooner); the
                                     forward queue (p2r_queue.flags): the same per chunk of an item;
                                     p2r_forward_backward (cfg.flags): within windows of 512 tracks of
                                     each event, 4 bytes of workspace per track; the queue adjoint

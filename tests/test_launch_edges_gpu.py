@@ -77,3 +77,25 @@ def test_dependent_launches_under_capture():
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(bits(out), bits(want))
+
+
+# below, at and above the size from which a masked batch is ordered (12 groups of 32 tracks per SM)
+@pytest.mark.parametrize("groups", [1, 12 * 148 - 1, 12 * 148, 12 * 148 + 1, 16 * 148 + 5])
+@pytest.mark.parametrize("bsize,options", [(32, False), (64, True), (256, False)])
+def test_ordered_flag_around_its_line(groups, bsize, options):
+    import p2r_tests_b200 as p2r
+    p2r, torch, cfg, trk, hit = make(bsize, max(1, groups * 32 // bsize), 1, 5)
+    if options:
+        cfg.flags = p2r.FLAG_SQUASH_PHI
+    nlay = torch.randint(0, 7, (cfg.ntracks,), dtype=torch.int32, device="cuda")  # 6: more than there are
+    dr = torch.linspace(-0.01, 0.01, 5, device="cuda") if options else None
+    outs = []
+    for flag in (0, p2r.FLAG_ORDER_BY_LAYERS):
+        cfg.flags = (cfg.flags & ~p2r.FLAG_ORDER_BY_LAYERS) | flag
+        for threads in (0, 128):
+            cfg.block_threads = threads
+            out, chi2 = torch.empty_like(trk), torch.empty(cfg.ntracks, device="cuda")
+            p2r.forward(cfg, trk, hit, out, chi2=chi2, dr=dr, nlay_lane=nlay)
+            outs.append((bits(out), bits(chi2)))
+    for o, c in outs[1:]:
+        assert np.array_equal(o, outs[0][0]) and np.array_equal(c, outs[0][1])
