@@ -235,13 +235,13 @@ __global__ void __launch_bounds__(kAdjThreads) fwdbwd_kernel(AdjParams p) {
 // buffer, and reverses the layers. At CK = 1 every layer has a slot, and the slot holds the
 // propagated state entering the layer's update instead: the reverse starts each layer from it
 // and rebuilds the layer's input with one update of the previous slot. Layout of both:
-// [slot][27 components][thread], so a warp's 32 lanes read and write one 256-byte (double) or
+// [slot][warp][27 components][32 lanes], so a warp's 32 lanes read and write one 256-byte (double) or
 // 128-byte (float) line per component. Used when the caller's workspace holds the tape
 // (p2r_forward_backward_workspace_size_tape).
 struct TapeParams {
-  void* tape;      // [nslots][27][nthreads] of T: the state before layers 0, CK, 2 CK, ...;
+  void* tape;      // [nslots][warps][27][32] of T: the state before layers 0, CK, 2 CK, ...;
                    // for CK = 1 the state after each layer's propagation, entering its update
-  void* segbuf;    // [CK - 1][27][nthreads] of T: the state before layers a+1 .. a+CK-1
+  void* segbuf;    // [CK - 1][warps][27][32] of T: the state before layers a+1 .. a+CK-1
   long long nthreads;
 };
 
@@ -265,6 +265,14 @@ struct TapeRef {
     for (int i = 0; i < 21; ++i) cov[i] = q[(6 + i) * comp];
   }
 };
+
+// Thread g's column of a grid tape: [slot][warp][27 components][32 lanes], so that the components of a
+// warp's tracks are 27 lines in a row at distances known to the compiler (with [slot][27][thread] each
+// of the 54 loads of a layer formed its own 64-bit address: 9600 x 100 x 20 tracks 4.77 -> 4.71 ms).
+template <class T>
+__device__ __forceinline__ TapeRef<T> tape_column(void* base, long long nthreads, long long g) {
+  return TapeRef<T>{(T*)base, 27 * nthreads, 32, (g >> 5) * (27 * 32) + (g & 31)};
+}
 
 // Per-track set-up shared by the tape kernels and the queue kernel: track (block b, lane it)
 // of the Matriplex arrays, its initial state, layer count and k = q kfact.
@@ -483,14 +491,21 @@ __device__ __forceinline__ void rev_track_ck1(const AdjParams& p, const TrackCtx
   finish_track(p, c, pb, cb, kbar, kinvbar, wpart);
 }
 
-template <class T, int CK>
-__global__ void __launch_bounds__(kAdjThreads) fwd_tape_kernel(AdjParams p, TapeParams tp) {
+// BS: the block width, compiled in (0: at run time), so that the hit rows lie at distances the loads carry
+// as immediates (9600 x 100 x 20 tracks at stride 1: 4.71 -> 4.67 ms). The reverse and the queue kernel
+// keep it at run time, although they would gain 4 and 6 %: there the compiler then fuses other products
+// into sums than it does now, and the two kernels, and each and its earlier builds, no longer agree to
+// the last bit, which ill-conditioned tracks amplify (one in 1e5 by 1e10).
+template <class T, int CK, int BS>
+__global__ void __launch_bounds__(kAdjThreads) fwd_tape_kernel(AdjParams args, TapeParams tp) {
   pdl_wait();
+  AdjParams p = args;
+  if (BS > 0) p.bsize = BS;
   T par[6], cov[21];
   long long g;
   const TrackCtx<T> c = grid_track(p, par, cov, g);
   const int bs = p.bsize;
-  const TapeRef<T> tr{(T*)tp.tape, 27 * tp.nthreads, tp.nthreads, g};
+  const TapeRef<T> tr = tape_column<T>(tp.tape, tp.nthreads, g);
   if constexpr (CK == 1) {
     fwd_track_ck1(p, c, par, cov, tr);
   } else {
@@ -512,12 +527,12 @@ __global__ void __launch_bounds__(kAdjThreads) rev_tape_kernel(AdjParams p, Tape
   long long g;
   const TrackCtx<T> c = grid_track(p, par, cov, g);
   const int bs = p.bsize;
-  const TapeRef<T> tr{(T*)tp.tape, 27 * tp.nthreads, tp.nthreads, g};
+  const TapeRef<T> tr = tape_column<T>(tp.tape, tp.nthreads, g);
   double* wpart = p.partials + (g >> 5) * (p.nlayer + 1);
   if constexpr (CK == 1) {
     rev_track_ck1(p, c, tr, wpart);
   } else {
-    const TapeRef<T> sr{(T*)tp.segbuf, 27 * tp.nthreads, tp.nthreads, g};
+    const TapeRef<T> sr = tape_column<T>(tp.segbuf, tp.nthreads, g);
     T pb[6], cb[21], chi2b;
     load_seeds(p, c, pb, cb, chi2b);
     T kbar = 0, kinvbar = 0;
@@ -803,8 +818,8 @@ WsLayout layout_of(const p2r_config* cfg) {
   return w;
 }
 
-// Tape region after the partial sums: [nslots][27][nthreads] checkpoints, then
-// [CK - 1][27][nthreads] segment states, in the kernel's arithmetic type.
+// Tape region after the partial sums: [nslots][warps][27][32] checkpoints, then
+// [CK - 1][warps][27][32] segment states, in the kernel's arithmetic type.
 struct TapeLayout {
   long long nthreads;
   size_t tape_off, seg_off, end;
@@ -827,7 +842,9 @@ int normal_ckpt(int ckpt_stride) { return ckpt_stride == 0 ? 5 : ckpt_stride; }
 template <class T, int CK>
 cudaError_t launch_tape(const AdjParams& p, const TapeParams& tp, cudaStream_t st) {
   const dim3 grid((unsigned)(tp.nthreads / kAdjThreads));
-  const cudaError_t e = launch_pdl(fwd_tape_kernel<T, CK>, grid, kAdjThreads, 0, st, p, tp);
+  auto fwd = fwd_tape_kernel<T, CK, 0>;
+  if constexpr (CK == 1) fwd = p.bsize == 32 ? fwd_tape_kernel<T, CK, 32> : fwd;
+  const cudaError_t e = launch_pdl(fwd, grid, kAdjThreads, 0, st, p, tp);
   return e != cudaSuccess ? e : launch_pdl(rev_tape_kernel<T, CK>, grid, kAdjThreads, 0, st, p, tp);
 }
 
