@@ -1293,9 +1293,7 @@ int enqueue_queue_adjoint(const p2r_queue* q, const void* trk_in, const void* hi
   qp.tapes = (double*)((char*)workspace + w.tape_off);
   qp.order = (q->flags & P2R_FLAG_ORDER_BY_LAYERS) ? (const uint32_t*)((char*)workspace + w.order_off) : nullptr;
   // counter and error word cleared; slice partials zeroed (slices of skipped items add nothing)
-  cudaError_t e = cudaMemsetAsync(workspace, 0, 256, st);
-  if (e == cudaSuccess && w.nslices > 0)
-    e = cudaMemsetAsync(qp.slice_partials, 0, (size_t)w.nslices * (q->nlayer + 1) * sizeof(double), st);
+  cudaError_t e = cudaMemsetAsync(workspace, 0, w.partial_off + (size_t)w.nslices * (q->nlayer + 1) * sizeof(double), st);
   if (e == cudaSuccess && qp.order && q->nblocks > 0) {
     e = launch_pdl(order_by_layers_kernel, order_grid(q->nevts), kOrderThreads, 0, st, q->nlay_lane,
                    q->event_block_offset, 0LL, q->nblocks, q->bsize, q->nlayer, 0LL, (uint32_t*)qp.order);

@@ -12,16 +12,20 @@
 namespace p2r {
 
 // ---------------------------------------------------------------- per-layer kernels
-// At 96000 tracks a launch moves 21 MB between L2 and the SMs and takes 4.8 us (B200), most of it one
-// track's latency. Capping the registers so that all 750 CTAs are resident at once (6 per SM, 80
-// registers, 120 bytes of spills) is slower: the loop of 40 launches takes 244 us, at 5 per SM 214 us,
-// uncapped (126 registers) 190 us. At 960000 tracks the two launches take 45 and 39 us, near the time
-// of their DRAM traffic (34 and 38 us).
+// At 96000 tracks a launch moves 21 MB between L2 and the SMs and takes 3.6 us (B200), most of it one
+// track's latency; at 960000 tracks the two launches take 35 and 38 us, the time of their DRAM traffic
+// (34 and 38 us). The block width BS is compiled in (0: at run time), so that the 30 rows read and 28
+// written lie at distances the loads and stores carry as immediates: 64 registers instead of 126, 24
+// warps per SM instead of 16, the loop of 40 launches 186 -> 144 us, the large propagation 45 -> 35 us.
+// Capping the registers of the run-time form at 80 or 96 instead spills: 244 and 214 us.
 constexpr int kLayerThreads = 128;
+
+template <int BS>
 __global__ void __launch_bounds__(kLayerThreads) propagate_kernel(const float* trk_in, const float* hits, float* trk_out,
-                                                        const float* dr, long long nblocks, int bs, int nlayer,
-                                                        int layer, float kfact) {
+                                                                  const float* dr, long long nblocks, int bsize,
+                                                                  int nlayer, int layer, float kfact) {
   pdl_wait();
+  const int bs = BS > 0 ? BS : bsize;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long b = g / bs;
   const int it = (int)(g - b * bs);
@@ -48,10 +52,12 @@ __global__ void __launch_bounds__(kLayerThreads) propagate_kernel(const float* t
   ob[27 * bs + it] = qf;
 }
 
-template <bool FP64DET>
-__global__ void __launch_bounds__(kLayerThreads) update_kernel(float* trk, const float* hits, float* chi2_accum, long long nblocks,
-                                                     int bs, int nlayer, int layer, int squash) {
+template <bool FP64DET, int BS>
+__global__ void __launch_bounds__(kLayerThreads) update_kernel(float* trk, const float* hits, float* chi2_accum,
+                                                               long long nblocks, int bsize, int nlayer, int layer,
+                                                               int squash) {
   pdl_wait();
+  const int bs = BS > 0 ? BS : bsize;
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long b = g / bs;
   const int it = (int)(g - b * bs);
@@ -80,6 +86,25 @@ __global__ void __launch_bounds__(kLayerThreads) update_kernel(float* trk, const
 #pragma unroll
   for (int i = 0; i < 21; ++i) blk[(6 + i) * bs + it] = cov[i];
   if (chi2_accum) chi2_accum[b * bs + it] += chi2;
+}
+
+// The per-layer kernels of a block width.
+auto propagate_for(int bsize) {
+  switch (bsize) {
+    case 32: return propagate_kernel<32>;
+    case 64: return propagate_kernel<64>;
+    case 128: return propagate_kernel<128>;
+    default: return propagate_kernel<0>;
+  }
+}
+template <bool FP64DET>
+auto update_for(int bsize) {
+  switch (bsize) {
+    case 32: return update_kernel<FP64DET, 32>;
+    case 64: return update_kernel<FP64DET, 64>;
+    case 128: return update_kernel<FP64DET, 128>;
+    default: return update_kernel<FP64DET, 0>;
+  }
 }
 
 __global__ void count_nonfinite_kernel(const float* trk, long long nblocks, int bs, unsigned long long* count) {
@@ -222,7 +247,7 @@ int p2r_propagate_to_r(const p2r_config* cfg, const void* trk_in, const void* hi
   const long long ntr = nblocks * cfg->bsize;
   const dim3 grid((unsigned)((ntr + kLayerThreads - 1) / kLayerThreads));
   const cudaError_t e =
-      launch_pdl(propagate_kernel, grid, kLayerThreads, 0, (cudaStream_t)stream, (const float*)trk_in, (const float*)hits,
+      launch_pdl(propagate_for(cfg->bsize), grid, kLayerThreads, 0, (cudaStream_t)stream, (const float*)trk_in, (const float*)hits,
                  (float*)trk_out, dr, nblocks, cfg->bsize, cfg->nlayer, layer, p2r_kfact_of(cfg->bz));
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "p2r_propagate_to_r: %s", cudaGetErrorString(e));
   return p2r_clear_error();
@@ -250,8 +275,8 @@ int p2r_kalman_update(const p2r_config* cfg, void* trk, const void* hits, int32_
   const dim3 grid((unsigned)((ntr + kLayerThreads - 1) / kLayerThreads));
   const int squash = (cfg->flags & P2R_FLAG_SQUASH_PHI) != 0;
   const cudaError_t e =
-      launch_pdl((cfg->flags & P2R_FLAG_FP32_DET) ? update_kernel<false> : update_kernel<true>, grid, kLayerThreads, 0,
-                 (cudaStream_t)stream, (float*)trk, (const float*)hits, chi2_accum, nblocks, cfg->bsize, cfg->nlayer, layer,
+      launch_pdl((cfg->flags & P2R_FLAG_FP32_DET) ? update_for<false>(cfg->bsize) : update_for<true>(cfg->bsize), grid,
+                 kLayerThreads, 0, (cudaStream_t)stream, (float*)trk, (const float*)hits, chi2_accum, nblocks, cfg->bsize, cfg->nlayer, layer,
                  squash);
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "p2r_kalman_update: %s", cudaGetErrorString(e));
   return p2r_clear_error();
