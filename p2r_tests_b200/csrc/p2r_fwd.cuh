@@ -208,12 +208,18 @@ __global__ void __launch_bounds__(128) fwd_kernel(FwdParams p) {
   } else {
     // Any bsize and alignment: a lane reads its own track's hits, the next layer's in flight while the
     // current one computes (loaded at the top of each layer instead, 400000 tracks x 20 layers at bsize
-    // 20 take 198 us, so 195; 160 tracks 20.6 -> 18.5 us: B200).
+    // 20 take 198 us, so 195; 160 tracks 20.6 -> 18.5 us: B200). One pointer steps through the rows by
+    // their width: nine addresses formed from the row number take registers from the arithmetic (86060
+    // tracks x 17 layers at bsize 20, chi2, offsets and wrapped phi: 45.3 -> 41.4 us).
     const float* h = hblk + it;
+    const unsigned bs4 = 4u * bs;
     float hn[9];
     if (nl > 0) {
 #pragma unroll
-      for (int i = 0; i < 9; ++i) hn[i] = __ldcs(h + i * bs);
+      for (int i = 0; i < 9; ++i) {
+        hn[i] = __ldcs(h);
+        h = (const float*)((const char*)h + bs4);
+      }
     }
     for (int l = 0; l < nl; ++l) {
       float hp[3], hc[6];
@@ -222,9 +228,11 @@ __global__ void __launch_bounds__(128) fwd_kernel(FwdParams p) {
 #pragma unroll
       for (int i = 0; i < 6; ++i) hc[i] = hn[3 + i];
       if (l + 1 < nl) {  // the next layer's hit, in flight while this layer computes
-        h += kHitWords * bs;
 #pragma unroll
-        for (int i = 0; i < 9; ++i) hn[i] = __ldcs(h + i * bs);
+        for (int i = 0; i < 9; ++i) {
+          hn[i] = __ldcs(h);
+          h = (const float*)((const char*)h + bs4);
+        }
       }
       const float rh = hipo(hp[0], hp[1]);
       const float rt = DR ? rh + __ldg(p.dr + l) : rh;
