@@ -13,7 +13,7 @@ __global__ void __launch_bounds__(NW * 32, kOrdWarpsPerSm / NW) fwd_ordered_kern
   const int cb = ordered_chunk_blocks<NW>(bs);
   const long long b0 = (long long)blockIdx.x * cb;
   const int nblk = (int)(p.nblocks - b0 < cb ? p.nblocks - b0 : cb);
-  ordered_chunk<BS, NW, CHI2, DR, true, SQUASH>(p, b0, nblk, sm);
+  ordered_chunk<BS, NW, CHI2, DR, true, SQUASH, CHI2>(p, b0, nblk, sm);
 }
 
 template <int BS, int NW, bool CHI2, bool DR, bool SQUASH>

@@ -44,7 +44,11 @@ __host__ __device__ __forceinline__ int ordered_chunk_blocks(int bsize) {
 
 // Runs blocks [b0, b0 + nblk) (nblk <= ordered_chunk_blocks<NW>(bsize)) with all NW warps of the
 // CTA; returns after a barrier, when the shared memory may be reused.
-template <int BS, int NW, bool CHI2, bool DR, bool FP64DET, bool SQUASH>
+// kStep: the hit pointer steps from layer to layer; otherwise each layer's address is formed from its
+// number. With one chunk per CTA and chi2 it is faster (1e6 tracks x 20-40 layers, B200: 742 -> 727 us;
+// bsize 128 737 -> 725), without chi2 not (706 -> 711 us), nor in the queue's loop over chunks (1000
+// events, 10-25 layers: 1340 -> 1363 us). Same bits.
+template <int BS, int NW, bool CHI2, bool DR, bool FP64DET, bool SQUASH, bool kStep>
 __device__ __forceinline__ void ordered_chunk(const FwdParams& p, long long b0, int nblk, OrdSmem<NW>& sm) {
   constexpr int kThreads = NW * 32;
   const int bs = BS > 0 ? BS : p.bsize;
@@ -119,6 +123,7 @@ __device__ __forceinline__ void ordered_chunk(const FwdParams& p, long long b0, 
 #pragma unroll
       for (int i = 0; i < 9; ++i) hn[i] = __ldg(hb + i * bs);
     }
+    if (kStep) hb += lstride;
     for (int l = 0; l < nl; ++l) {
       float hp[3], hc[6];
 #pragma unroll
@@ -127,7 +132,8 @@ __device__ __forceinline__ void ordered_chunk(const FwdParams& p, long long b0, 
       for (int i = 0; i < 6; ++i) hc[i] = hn[3 + i];
       if (l + 1 < nl) {  // the next layer's hit, in flight while this layer computes
 #pragma unroll
-        for (int i = 0; i < 9; ++i) hn[i] = __ldg(hb + (l + 1) * lstride + i * bs);
+        for (int i = 0; i < 9; ++i) hn[i] = __ldg((kStep ? hb : hb + (l + 1) * lstride) + i * bs);
+        if (kStep) hb += lstride;
       }
       const float rh = hipo(hp[0], hp[1]);
       const float rt = DR ? rh + __ldg(p.dr + l) : rh;

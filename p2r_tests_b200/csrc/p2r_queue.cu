@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(NW * 32, kOrdWarpsPerSm / NW) queue_ordered_ke
     }
     for (int c0 = 0; c0 < qi.nblk; c0 += cb) {
       const int nblk = min(cb, qi.nblk - c0);
-      ordered_chunk<BS, NW, CHI2, false, FP64DET, SQUASH>(p, qi.block0 + c0, nblk, sm);
+      ordered_chunk<BS, NW, CHI2, false, FP64DET, SQUASH, false>(p, qi.block0 + c0, nblk, sm);
       if (tid == 0) {
         __threadfence();
         if (atomicSub(&q.ev_remaining[qi.event], nblk * spb) == nblk * spb && q.ev_done)
