@@ -56,6 +56,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return r;
 }
 #if defined(P2R_FAST_MATH)
+__device__ __forceinline__ float frcp(float b) { return __fdividef(1.f, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float fsqrt(float x) {
   float r;
@@ -77,6 +78,7 @@ __device__ __forceinline__ float fsqrt(float x) {
   return ffma(fmul(0.5f, r), ffma(-s, s, x), s);
 }
 #else
+__device__ __forceinline__ float frcp(float b) { return __fdiv_rn(1.f, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ float fsqrt(float x) { return __fsqrt_rn(x); }
 #endif
@@ -139,16 +141,18 @@ __device__ __forceinline__ float mulcos(float v, float omc) { return ffma(-v, om
 // Propagates (ip, ic) to the cylinder of radius r. k = q*kfact, kinv = 1/k.
 // op/oc may be the same arrays as ip/ic: every input is read before any output is written.
 // kEarly: each helix iteration starts the next one's reciprocal root before it forms its path
-// derivatives, whose branch the compiler does not move it across. Same operations, same bits. Chained
-// fused forward (B200) of 19200 x 20 tracks 23.2 -> 22.4 us, of 960000 x 20 431.1 -> 429.8 us; with
-// lanes masked out it is slower (1e6 tracks x 20-40 layers in generator order 901 -> 921 us).
+// derivatives, whose branch the compiler does not move it across, and a reciprocal is taken as such,
+// where fdiv(1, b) leaves a product by 1 in the code. Same bits. Chained fused forward (B200) of 19200
+// x 20 tracks 23.2 -> 22.3 us, of 960000 x 20 431.1 -> 429.8 -> 427.1 us; with lanes masked out both are
+// slower (1e6 tracks x 20-40 layers in generator order 901 -> 921 and 906 us).
 template <bool kEarly = false>
 __device__ __forceinline__ void propagate_to_r(const float (&ip)[6], const float (&ic)[21], float k, float kinv,
                                                float r, float (&op)[6], float (&oc)[21]) {
   const float xin = ip[0], yin = ip[1], zin = ip[2];
   const float iptin = ip[3], phiin = ip[4], thetain = ip[5];
+  auto inv = [](float b) { return kEarly ? frcp(b) : fdiv(1.f, b); };
   float r0 = hipo(xin, yin);
-  const float pt = fdiv(1.f, iptin);
+  const float pt = inv(iptin);
   const float ik = fmul(iptin, kinv);  // turning angle per unit of path length
   const float kpt = fmul(k, pt);
 
@@ -185,7 +189,7 @@ __device__ __forceinline__ void propagate_to_r(const float (&ip)[6], const float
     // derivative increment by oor0 = 0 until then; adding a finite x * 0 leaves the sums
     // unchanged, so those increments are skipped.
     if (i + 1 != 5 && r0 > 0.f && fabsf(id) < 0.0001f) {
-      const float noor0 = -fdiv(1.f, r0);  // -1/r0
+      const float noor0 = -inv(r0);  // -1/r0
       const float kn = fmul(iptin, noor0);  // k*dadx/xo = k*dady/yo of TBB:716-717
       // dDdx -= (xo*(1 + tx*a1) + yo*tx*a2) * oor0 and dDdy -= (xo*ty*a1 + yo*(1 + ty*a2)) * oor0
       // with tx = kn*xo, ty = kn*yo: xo resp. yo times (1 + kn*(xo*a1 + yo*a2)) * oor0
@@ -242,7 +246,7 @@ __device__ __forceinline__ void propagate_to_r(const float (&ip)[6], const float
   const float J14 = fmul(ffma(dadphi, sc, ffma(cosP, sina, fmul(-sinP, omc))), kpt);
   float sinT, cosT;
   sincosf(thetain, &sinT, &cosT);  // theta can be large: no approximation (TBB:767-769)
-  const float isinT = fdiv(1.f, sinT);
+  const float isinT = inv(sinT);
   const float kpi = fmul(kpt, isinT);  // k*pt/sinT
   const float kpc = fmul(kpi, cosT);   // k*pt*cosT/sinT
   // rows 2 and 4 share (dadx, dady, ., ., dadphi, .): J2 = kpc*(dadx, dady, 0, 0, dadphi, 0)
