@@ -27,7 +27,9 @@ inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t
   c.stream = st;
   c.attrs = &at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kern, (P)args...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kern, (P)args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported once: nothing stays pending
+  return e;
 }
 
 }  // namespace p2r
