@@ -152,12 +152,15 @@ def run_layers(cfg: Config, trk_in, hits, trk_out, stream=None) -> None:
     (96000 tracks, where a kernel takes 4 to 5), 8 were spent on that. The first layer reads trk_in
     itself where that is all the copy trk_out.copy_(trk_in) would amount to (_same_as_copied);
     anything else is copied."""
+    from torch.autograd.graph import increment_version
     restart = cfg.mode == MODE_RESTART
     _check_shapes(cfg, trk_out, hits)
     if restart:
         _check_shapes(cfg, trk_in, None)
     direct = _same_as_copied(trk_in, trk_out)
-    if cfg.nlayer < 1 or not direct:
+    if cfg.nlayer >= 1 and direct:
+        increment_version(trk_out)  # as torch's copy does: a backward pass that saved trk_out has to see the write
+    else:
         trk_out.copy_(trk_in)
     c = ctypes.byref(cfg.c())
     p_out, p_hits, st = _ptr(trk_out), _ptr(hits), _stream(stream)
@@ -173,11 +176,13 @@ def run_layers(cfg: Config, trk_in, hits, trk_out, stream=None) -> None:
 
 def _same_as_copied(src, dst) -> bool:
     """Whether dst.copy_(src) would do no more than copy src's bytes to dst: one shape, type and
-    device, plain memory that the two do not share."""
+    device, plain memory that the two do not share, and nothing for autograd to refuse or record."""
     import torch
     if not (type(src) is torch.Tensor and type(dst) is torch.Tensor and src.shape == dst.shape
             and src.dtype == dst.dtype and src.device == dst.device and src.is_contiguous()
-            and torch._C._has_storage(src) and not src.is_neg()):
+            and torch._C._has_storage(src) and not src.is_neg() and not src.requires_grad
+            and not dst.requires_grad and not dst.is_inference()
+            and torch.autograd.forward_ad._current_level < 0):
         return False
     x, y, n = src.data_ptr(), dst.data_ptr(), src.nbytes
     return x != 0 and (x + n <= y or y + n <= x)

@@ -81,3 +81,35 @@ def test_converted_forms_are_copied(loop, form):
     loop(src, out)
     assert loop.calls[0][1] == out.data_ptr()
     assert torch.equal(out, want)
+
+
+def test_the_write_is_seen_by_autograd(loop):
+    t, out = tracks(), torch.zeros(2, 28, 4)
+    before = out._version
+    loop(t, out)
+    assert out._version > before
+    w = torch.ones(2, 28, 4, requires_grad=True)
+    loss = (w * out).sum()
+    loop(t, out)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
+
+
+def test_autograd_refuses_and_records_as_the_copy_does(loop):
+    with pytest.raises(RuntimeError):
+        loop(tracks(), torch.zeros(2, 28, 4, requires_grad=True))
+    out = torch.zeros(2, 28, 4)
+    loop(tracks().requires_grad_(), out)
+    assert out.requires_grad
+    with torch.inference_mode():
+        out = torch.zeros(2, 28, 4)
+    with pytest.raises(RuntimeError):
+        loop(tracks(), out)
+
+
+def test_forward_mode_tangent_goes_with_the_copy(loop):
+    import torch.autograd.forward_ad as fwd
+    out = torch.zeros(2, 28, 4)
+    with fwd.dual_level():
+        loop(fwd.make_dual(tracks(), torch.ones(2, 28, 4)), out)
+        assert torch.equal(fwd.unpack_dual(out).tangent, torch.ones(2, 28, 4))
