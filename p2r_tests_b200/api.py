@@ -153,12 +153,15 @@ def run_layers(cfg: Config, trk_in, hits, trk_out, stream=None) -> None:
     itself where that is all the copy trk_out.copy_(trk_in) would amount to (_same_as_copied);
     anything else is copied."""
     from torch.autograd.graph import increment_version
+    if cfg.nlayer < 1:
+        trk_out.copy_(trk_in)
+        return
     restart = cfg.mode == MODE_RESTART
     _check_shapes(cfg, trk_out, hits)
     if restart:
         _check_shapes(cfg, trk_in, None)
     direct = _same_as_copied(trk_in, trk_out)
-    if cfg.nlayer >= 1 and direct:
+    if direct:
         increment_version(trk_out)  # as torch's copy does: a backward pass that saved trk_out has to see the write
     else:
         trk_out.copy_(trk_in)

@@ -113,3 +113,9 @@ def test_forward_mode_tangent_goes_with_the_copy(loop):
     with fwd.dual_level():
         loop(fwd.make_dual(tracks(), torch.ones(2, 28, 4)), out)
         assert torch.equal(fwd.unpack_dual(out).tangent, torch.ones(2, 28, 4))
+
+
+def test_no_layers_is_the_copy(loop, p2r):
+    t, out = tracks(), torch.zeros(2, 28, 4)
+    p2r.run_layers(p2r.Config(bsize=4, nlayer=0, nevts=1, nb=2), t, None, out)
+    assert torch.equal(out, t)
