@@ -151,8 +151,10 @@ def run_layers(cfg: Config, trk_in, hits, trk_out, stream=None) -> None:
     The arguments are checked and converted once, not once per call: of the 11.4 us a call took
     (96000 tracks, where a kernel takes 4 to 5), 8 were spent on that. The first layer reads trk_in
     itself where that is all the copy trk_out.copy_(trk_in) would amount to (_same_as_copied);
-    anything else is copied."""
-    from torch.autograd.graph import increment_version
+    anything else is copied. Copy and kernels run on `stream`, after what was queued there before, and
+    trk_in may be freed as soon as the call returns (restart mode on a bare stream handle: once that
+    stream is done, since every layer reads it)."""
+    import torch
     if cfg.nlayer < 1:
         trk_out.copy_(trk_in)
         return
@@ -160,14 +162,21 @@ def run_layers(cfg: Config, trk_in, hits, trk_out, stream=None) -> None:
     _check_shapes(cfg, trk_out, hits)
     if restart:
         _check_shapes(cfg, trk_in, None)
-    direct = _same_as_copied(trk_in, trk_out)
-    if direct:
-        increment_version(trk_out)  # as torch's copy does: a backward pass that saved trk_out has to see the write
-    else:
-        trk_out.copy_(trk_in)
-    c = ctypes.byref(cfg.c())
     p_out, p_hits, st = _ptr(trk_out), _ptr(hits), _stream(stream)
+    side = None if stream is None else _side_stream(stream, st, trk_out.device)
+    direct = _same_as_copied(trk_in, trk_out) and (side is None or side is stream)
+    if direct:
+        # as torch's copy does: a backward pass that saved trk_out has to see the write
+        torch.autograd.graph.increment_version(trk_out)
+    elif side is None:
+        trk_out.copy_(trk_in)
+    else:
+        with torch.cuda.stream(side):
+            trk_out.copy_(trk_in)
+    if side is not None and trk_in.device == trk_out.device:
+        _hold(trk_in, side, side is stream)
     src = _ptr(trk_in) if direct or restart else p_out
+    c = ctypes.byref(cfg.c())
     propagate, update = lib().p2r_propagate_to_r, lib().p2r_kalman_update
     for layer in range(cfg.nlayer):
         rc = propagate(c, src, p_hits, layer, p_out, None, st) or update(c, p_out, p_hits, layer, None, st)
@@ -175,6 +184,35 @@ def run_layers(cfg: Config, trk_in, hits, trk_out, stream=None) -> None:
             check(rc)
         if not restart:
             src = p_out
+
+
+def _side_stream(stream, handle: int, device):
+    """None where `stream` is torch's current stream of `device`, else a torch stream object for it:
+    `stream` itself if it is one, or one made from its handle."""
+    import torch
+    handle = 0 if handle == 1 else handle  # cudaStreamLegacy
+    if handle == torch.cuda.current_stream(device).cuda_stream:
+        return None
+    return stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(handle, device=device)
+
+
+def _hold(t, side, owned: bool) -> None:
+    """Keeps t's memory from being reused while `side` reads it. A torch stream is named to the
+    allocator. A bare handle may be gone when t is freed, so there the current stream waits for what
+    `side` holds so far; not while either is captured, where such a wait would join the two."""
+    import torch
+    if owned:
+        t.record_stream(side)
+        return
+    capturing = torch.cuda.is_current_stream_capturing
+    if capturing():
+        return
+    current = torch.cuda.current_stream(t.device)
+    with torch.cuda.stream(side):
+        if capturing():
+            return
+        done = side.record_event()
+    current.wait_event(done)
 
 
 def _same_as_copied(src, dst) -> bool:

@@ -119,3 +119,100 @@ def test_no_layers_is_the_copy(loop, p2r):
     t, out = tracks(), torch.zeros(2, 28, 4)
     p2r.run_layers(p2r.Config(bsize=4, nlayer=0, nevts=1, nb=2), t, None, out)
     assert torch.equal(out, t)
+
+
+class FakeStreams:
+    """torch.cuda's stream calls over handles: the current stream is 0; `log` takes what happens where."""
+
+    class Stream:
+        def __init__(self, handle, device=None):
+            self.cuda_stream = handle
+
+    def __init__(self, monkeypatch):
+        from p2r_tests_b200 import api
+        self.log, self.now, self.captured = [], self.Stream(0), set()
+        cuda = torch.cuda
+
+        class On:
+            def __init__(ctx, s):
+                ctx.s = s
+
+            def __enter__(ctx):
+                ctx.before, self.now = self.now, ctx.s
+
+            def __exit__(ctx, *exc):
+                self.now = ctx.before
+
+        copy, record = torch.Tensor.copy_, self.log.append
+        self.Stream.record_event = lambda s: (record(("event", s.cuda_stream)), s.cuda_stream)[1]
+        self.Stream.wait_event = lambda s, e: record(("wait", s.cuda_stream, e))
+        monkeypatch.setattr(cuda, "Stream", self.Stream)
+        monkeypatch.setattr(cuda, "ExternalStream", self.Stream)
+        monkeypatch.setattr(cuda, "stream", On)
+        monkeypatch.setattr(cuda, "current_stream", lambda device=None: self.now)
+        monkeypatch.setattr(cuda, "is_current_stream_capturing", lambda: self.now.cuda_stream in self.captured)
+        monkeypatch.setattr(torch.Tensor, "copy_",
+                            lambda t, src: (record(("copy", self.now.cuda_stream)), copy(t, src))[1], raising=False)
+        monkeypatch.setattr(torch.Tensor, "record_stream",
+                            lambda t, s: record(("used", s.cuda_stream)), raising=False)
+        monkeypatch.setattr(api, "_stream", lambda s: s.cuda_stream if hasattr(s, "cuda_stream") else int(s or 0))
+
+
+@pytest.mark.parametrize("form,kind,expected", [
+    ("plain", "current", []),
+    ("plain", "legacy handle", []),
+    ("plain", "torch", [("used", 640)]),
+    ("plain", "handle", [("copy", 640), ("event", 640), ("wait", 0, 640)]),
+    ("strided", "current", [("copy", 0)]),
+    ("strided", "torch", [("copy", 640), ("used", 640)]),
+    ("strided", "handle", [("copy", 640), ("event", 640), ("wait", 0, 640)]),
+    ("strided", "captured handle", [("copy", 640)]),
+    ("strided", "handle under capture", [("copy", 640)]),
+])
+def test_copy_and_lifetime_on_another_stream(loop, p2r, monkeypatch, form, kind, expected):
+    """The copy belongs to the kernels' stream: on torch's current one it races with the first layer."""
+    fake = FakeStreams(monkeypatch)
+    t, out = tracks(), torch.zeros(2, 28, 4)
+    if form == "strided":
+        t = torch.stack([t, t], -1)[..., 0]
+    stream = {"current": fake.now, "legacy handle": 1, "torch": fake.Stream(640)}.get(kind, 640)
+    fake.captured = {"captured handle": {640}, "handle under capture": {0}}.get(kind, set())
+    fake.log.clear()
+    p2r.run_layers(p2r.Config(bsize=4, nlayer=NLAYER, nevts=1, nb=2), t, torch.zeros(2 * NLAYER, 9, 4), out,
+                   stream=stream)
+    assert fake.log == expected and len(loop.calls) == NLAYER
+
+
+def gpu_case(p2r, mode):
+    cfg = p2r.Config(bsize=24, nlayer=5, nevts=2, nb=3, bz=3.8, mode=mode)
+    trk, hit = p2r.generate_helix(cfg, p2r.gen_params(bz=3.8, seed=12))
+    t, h = torch.from_numpy(trk).cuda(), torch.from_numpy(hit).cuda()
+    want = torch.empty_like(t)
+    p2r.forward(cfg, t, h, want)
+    torch.cuda.synchronize()
+    return cfg, t, h, want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "host", "strided", "broadcast"])
+@pytest.mark.parametrize("kind", ["torch", "handle"])
+def test_side_stream_that_holds_earlier_work(p2r, form, kind):
+    cfg, t, h, want = gpu_case(p2r, p2r.MODE_CHAINED)
+    if form == "broadcast":
+        t[:] = t[0].clone()
+        p2r.forward(cfg, t, h, want)
+        torch.cuda.synchronize()
+    src = {"plain": t.clone, "host": t.cpu, "strided": lambda: torch.stack([t, t], -1)[..., 0],
+           "broadcast": lambda: t[:1].clone()}[form]()
+    side, out = torch.cuda.Stream(), torch.empty_like(t)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)  # about 10 ms
+        out.fill_(5.0)  # earlier work on the side stream that writes the output
+    p2r.run_layers(cfg, src, h, out, stream=side if kind == "torch" else side.cuda_stream)
+    shape, on_gpu = src.shape, src.is_cuda
+    del src  # free at once: the next allocation of its size may not land in it before it is read
+    if on_gpu:
+        torch.full(shape, float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    assert torch.equal(out.view(torch.int32), want.view(torch.int32))
