@@ -360,6 +360,8 @@ int32_t p2r_math_variant(void);
  * quot[i] = a[i] / b[i], root[i] = sqrt(a[i]), for measuring their error against the
  * correctly rounded results. Device pointers, n >= 0. */
 int p2r_math_check(int64_t n, const float* a, const float* b, float* quot, float* root, void* stream);
+/* The same for the FP64 adjoint: inv[i] = 1 / a[i], root[i] = sqrt(a[i]). */
+int p2r_math_check64(int64_t n, const double* a, double* inv, double* root, void* stream);
 
 /* ---------------------------------------------------------------- host-side helpers */
 

@@ -290,6 +290,14 @@ def math_check(a, b, stream=None):
     return quot, root
 
 
+def math_check64(a, stream=None):
+    """The FP64 adjoint's own 1 / a and sqrt(a) on the device (a: float64 tensor)."""
+    import torch
+    inv, root = torch.empty_like(a), torch.empty_like(a)
+    check(lib().p2r_math_check64(a.numel(), _arg(a, "float64", None, "a"), _ptr(inv), _ptr(root), _stream(stream)))
+    return inv, root
+
+
 def count_nonfinite(trk, nblocks: int, bsize: int, stream=None) -> int:
     import torch
     cnt = torch.zeros(1, dtype=torch.int64, device=trk.device)

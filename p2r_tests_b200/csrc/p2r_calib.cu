@@ -4,6 +4,7 @@
 // is eliminated. FLOPs per launch = 2 * 32 * iters * blocks * threads (8 chains, 4 rounds).
 #include <cuda_runtime.h>
 
+#include "p2r_adjoint.cuh"
 #include "p2r_internal.h"
 #include "p2r_math.cuh"
 
@@ -90,6 +91,15 @@ __global__ void math_check_kernel(long long n, const float* __restrict__ a, cons
   }
 }
 
+// The FP64 adjoint's own 1 / a and sqrt(a), for the same purpose.
+__global__ void math_check64_kernel(long long n, const double* __restrict__ a, double* __restrict__ inv,
+                                    double* __restrict__ root) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    inv[i] = p2r::adj::rcp_(a[i]);
+    root[i] = p2r::adj::sqrt_(a[i]);
+  }
+}
+
 }  // namespace
 
 extern "C" int p2r_fp32x2_fma_probe(int64_t iters, int32_t blocks, int32_t threads, float* out, void* stream) {
@@ -121,6 +131,18 @@ extern "C" int p2r_math_check(int64_t n, const float* a, const float* b, float* 
   math_check_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(n, a, b, quot, root);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "p2r_math_check: %s", cudaGetErrorString(e));
+  return p2r_clear_error();
+}
+
+extern "C" int p2r_math_check64(int64_t n, const double* a, double* inv, double* root, void* stream) {
+  if (n < 0 || (n > 0 && (!a || !inv || !root)))
+    return p2r_set_error(P2R_ERR_INVALID, "p2r_math_check64: bad arguments");
+  if (int rc = p2r_check_aligned("p2r_math_check64", 8, {a, inv, root})) return rc;
+  if (n == 0) return p2r_clear_error();
+  const long long blocks = (n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16;
+  math_check64_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(n, a, inv, root);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return p2r_set_errorf(P2R_ERR_CUDA, "p2r_math_check64: %s", cudaGetErrorString(e));
   return p2r_clear_error();
 }
 
