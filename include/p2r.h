@@ -157,7 +157,7 @@ int p2r_count_nonfinite(const void* trk, int64_t nblocks, int32_t bsize, unsigne
 
 /* Host-buffer driver: p2r_forward over HOST arrays (host_trk_in, host_hits -> host_trk_out)
  * through caller-provided device arrays of the full size. The track blocks are split into at
- * most nchunks contiguous chunks; each chunk's H2D copy, fused forward and D2H copy are queued on a
+ * most nchunks contiguous chunks (and at most one for every 4 MiB copied in); each chunk's H2D copy, fused forward and D2H copy are queued on a
  * library-owned pool of three streams so copies overlap kernels (the reference's
  * multi-stream driver, cuda_v4.cu:912-1010). Ordered after prior work on `stream`, and
  * `stream` waits for all of it. Host arrays should be pinned for the copies to overlap.

@@ -10,9 +10,11 @@
 // each track block is copied: one strided 2-D copy per chunk, a 1/nlayer share of the hits.
 //
 // The host link bounds the call (55.5 GB/s host->device); every gap between two copies and the last
-// chunk's kernel and copy back come on top. So chunks are equal numbers of blocks, but the last is a
-// quarter of the others; none is below 4 MiB, where a copy costs more than it hides; and in chained
-// mode the tracks (one byte in seven at 20 layers) go over in one copy before the hits.
+// chunk's kernel and copy back come on top. So chunks are equal numbers of blocks, but the last of three
+// or more is a quarter of the others; there is at most one for every 4 MiB of input, since smaller copies
+// cost more than they hide (a batch below 8 MiB is one chunk; the short last one may have a third of
+// 4 MiB); and in chained mode the tracks (one byte in seven at 20 layers) go over in one copy before the
+// hits.
 // Measured on one B200, pinned buffers, 8 chunks asked for, chunks of whole events before -> this:
 // 9600 x 10 x 20 1617 -> 1541 us (80 MB in, 1440 us at the link's rate), 9600 x 60 x 20 9.34 -> 8.83 ms,
 // 5000 x 7 x 12 470 -> 428 us, 9600 x 1 x 20 203 -> 201 us; restart 9600 x 10 505 -> 440 us. Tracks in
@@ -27,7 +29,7 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 constexpr int kPoolStreams = 3;
-constexpr size_t kMinChunkBytes = size_t(4) << 20;  // host->device bytes of a chunk
+constexpr size_t kMinChunkBytes = size_t(4) << 20;  // host->device bytes per chunk, on average
 constexpr int kLastShare = 4;                       // the last chunk is 1 / kLastShare of another
 
 struct StreamPool {
