@@ -37,10 +37,11 @@ def workspace_size(cfg: Config, ckpt_stride: int | None = None) -> int:
 
 def auto_ckpt_stride(cfg: Config, device, tape: bool = True) -> int:
     """The checkpoint stride used when the caller names none: 1 (the whole state tape, the
-    fastest reverse) when its workspace fits in half the free device memory, else 5; 5 for
-    thread-local checkpoints. A workspace of at most _SMALL_WORKSPACE is taken to fit: asking the
-    driver for the free memory takes 70 us, and 255 us while kernels run, as long as the whole
-    forward + adjoint of 9600 tracks."""
+    fastest reverse) when its workspace is at most _SMALL_WORKSPACE or fits in half the free
+    device memory, else 5; 5 for thread-local checkpoints. Up to _SMALL_WORKSPACE the free memory
+    is not asked for, however little there is (forward_backward takes stride 5 when the
+    workspace is refused): the question takes 70 us, and 255 us while kernels run, as long as
+    the whole forward + adjoint of 9600 tracks."""
     if not tape:
         return 5
     need = workspace_size(cfg, 1)
@@ -57,8 +58,9 @@ def forward_backward(cfg: Config, trk_in, hits, dr=None, nlay_lane=None, grad_tr
     tape: give the library a workspace that holds the checkpoint tape (two-kernel path);
     False keeps the checkpoints in thread-local memory (smallest workspace). ckpt_stride None:
     auto_ckpt_stride's choice, made once per `out` dict and kept with its workspace (so repeated
-    calls, a CUDA-graph capture among them, run the same stride). An entry of `out` set to None
-    skips that output (e.g. grad_hits for calibration-only runs)."""
+    calls, a CUDA-graph capture among them, run the same stride; 5 if the allocator refuses the
+    workspace of a stride 1 chosen so). An entry of `out` set to None skips that output (e.g.
+    grad_hits for calibration-only runs)."""
     _check_shapes(cfg, trk_in, hits)
     dev = trk_in.device
     o = out if out is not None else {}

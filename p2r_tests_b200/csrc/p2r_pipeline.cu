@@ -12,8 +12,8 @@
 // The host link bounds the call (55.5 GB/s host->device); every gap between two copies and the last
 // chunk's kernel and copy back come on top. So chunks are equal numbers of blocks, but the last of three
 // or more is a quarter of the others; there is at most one for every 4 MiB of input, since smaller copies
-// cost more than they hide (a batch below 8 MiB is one chunk; the short last one may have a third of
-// 4 MiB); and in chained mode the tracks (one byte in seven at 20 layers) go over in one copy before the
+// cost more than they hide (a batch below 8 MiB is one chunk; the short last one may have little over
+// 1 MiB); and in chained mode the tracks (one byte in seven at 20 layers) go over in one copy before the
 // hits.
 // Measured on one B200, pinned buffers, 8 chunks asked for, chunks of whole events before -> this:
 // 9600 x 10 x 20 1617 -> 1541 us (80 MB in, 1440 us at the link's rate), 9600 x 60 x 20 9.34 -> 8.83 ms,
