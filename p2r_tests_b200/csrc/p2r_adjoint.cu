@@ -492,7 +492,8 @@ __device__ __forceinline__ void rev_track_ck1(const AdjParams& p, const TrackCtx
 }
 
 // BS: the block width, compiled in (0: at run time), so that the hit rows lie at distances the loads carry
-// as immediates (9600 x 100 x 20 tracks at stride 1: 4.71 -> 4.67 ms). The reverse and the queue kernel
+// as immediates (960000 x 20 tracks at stride 1: 4.71 -> 4.67 ms). Compiled for 32, the default width; 64 and
+// 128 would go from 4.68 to 4.65 ms, too little for two more instances of each type. The reverse and the queue kernel
 // keep it at run time, although they would gain 4 and 6 %: there the compiler then fuses other products
 // into sums than it does now, and the two kernels, and each and its earlier builds, no longer agree to
 // the last bit, which ill-conditioned tracks amplify (one in 1e5 by 1e10).

@@ -133,7 +133,10 @@ static int check_ptr16(const void* ptr) { return ((uintptr_t)ptr & 15u) == 0; }
 // one group per warp, is done sooner; once warps queue for the SM partitions the lanes that ordering
 // keeps busy win. Measured on one B200 (148 SMs, 20-40 layers, ordered / unordered us): 9600 tracks
 // 51 / 37, 32000 52 / 49, 48000 73 / 62, 64000 74 / 79, 100000 96 / 114, 320000 264 / 299; 10-25 layers
-// cross at the same size. Both kernels give the same bits. The line: 12 groups of 32 tracks per SM.
+// cross at the same size. Without staging (P2R_FLAG_NO_STAGING, unaligned hits) the unordered kernel is 3 to
+// 10 % faster than with it and crosses at the same place: ordered / unordered 56832 tracks 72 / 61, 66304
+// 72 / 78, 94720 96 / 95, 151552 119 / 143. All kernels give the same bits. The line: 12 groups of 32
+// tracks per SM.
 static bool ordering_pays(long long ntr) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||

@@ -45,9 +45,10 @@ __host__ __device__ __forceinline__ int ordered_chunk_blocks(int bsize) {
 // Runs blocks [b0, b0 + nblk) (nblk <= ordered_chunk_blocks<NW>(bsize)) with all NW warps of the
 // CTA; returns after a barrier, when the shared memory may be reused.
 // kStep: the hit pointer steps from layer to layer; otherwise each layer's address is formed from its
-// number. With one chunk per CTA and chi2 it is faster (1e6 tracks x 20-40 layers, B200: 742 -> 727 us;
-// bsize 128 737 -> 725), without chi2 not (706 -> 711 us), nor in the queue's loop over chunks (1000
-// events, 10-25 layers: 1340 -> 1363 us). Same bits.
+// number. With one chunk per CTA and chi2 it is a little faster (1e6 tracks x 20-40 layers, B200, medians of
+// three runs: bsize 32 741 -> 724 us, 128 766 -> 767 to 785 -> 768, 64 no difference beyond noise; 10-25
+// layers 455 -> 451 us), without chi2 not (706 -> 711 us), nor in the queue's loop over chunks (1000 events,
+// 10-25 layers: 1340 -> 1363 us). Same bits.
 template <int BS, int NW, bool CHI2, bool DR, bool FP64DET, bool SQUASH, bool kStep>
 __device__ __forceinline__ void ordered_chunk(const FwdParams& p, long long b0, int nblk, OrdSmem<NW>& sm) {
   constexpr int kThreads = NW * 32;
