@@ -264,7 +264,7 @@ int p2r_graph_destroy(p2r_graph* g);
  * in double, so results are deterministic). With the checkpoints held per thread, the
  * kernel keeps them in thread-local memory; a workspace of
  * p2r_forward_backward_workspace_size_tape(cfg, ckpt_stride) bytes also holds them, and the
- * recomputed segment states, as a tape in device memory ([slot][27][thread], 27*(nlayer /
+ * recomputed segment states, as a tape in device memory ([slot][warp][27][32], 27*(nlayer /
  * ckpt_stride + ckpt_stride - 1) values per track), which runs the forward and the reverse
  * as two lighter kernels. Same results either way. */
 size_t p2r_forward_backward_workspace_size(const p2r_config* cfg);
