@@ -216,3 +216,18 @@ def test_side_stream_that_holds_earlier_work(p2r, form, kind):
         torch.full(shape, float("nan"), device="cuda")
     torch.cuda.synchronize()
     assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("handle", [0, 1, 2])  # the default stream: torch's, the legacy one by name, this thread's
+@pytest.mark.parametrize("form", ["plain", "strided"])
+def test_default_stream_handles(p2r, handle, form):
+    cfg, t, h, want = gpu_case(p2r, p2r.MODE_CHAINED)
+    src = t if form == "plain" else torch.stack([t, t], -1)[..., 0]
+    out, fused = torch.empty_like(t), torch.empty_like(t)
+    torch.cuda.synchronize()
+    p2r.run_layers(cfg, src, h, out, stream=handle)
+    p2r.forward(cfg, t, h, fused, stream=handle)
+    torch.cuda.synchronize()
+    assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+    assert torch.equal(fused.view(torch.int32), want.view(torch.int32))
